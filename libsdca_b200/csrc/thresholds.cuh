@@ -111,14 +111,15 @@ struct Taken {
   }
 };
 
-// Takes the largest entry not yet taken; false if none is left.
+// Takes the largest entry not yet taken; false if none is left.  NaN is never taken: no order holds
+// with it, and the lanes have to agree (warp_max).
 template <typename R, typename Row>
 SDCAB_D bool take_next(const Row& row, Taken<R>& tk, R& val) {
   R best = -num<R>::inf();
   int bi = INT_MAX;
   row.for_each([&](typename Row::data_type xd, int i) {
     R x = static_cast<R>(xd);
-    if (!tk.has(x, i) && (bi == INT_MAX || x > best)) { best = x; bi = i; }
+    if (!tk.has(x, i) && (x > best || (bi == INT_MAX && x == x))) { best = x; bi = i; }
   });
   // lanes without a candidate carry (-inf, INT_MAX) and lose every comparison
 #if defined(SDCAB_WARP_GROUP)
@@ -306,7 +307,7 @@ SDCAB_D Projection topk_special_cases(const Row& row, int k, R div, Thr<R>& thr)
   Taken<R> tk;
   R sum_k = 0, v_k = 0;
   for (int j = 0; j < k; ++j) {
-    R v;
+    R v = -num<R>::inf();
     take_next<R>(row, tk, v);
     sum_k += v; v_k = v;
   }
@@ -318,7 +319,7 @@ SDCAB_D Projection topk_special_cases(const Row& row, int k, R div, Thr<R>& thr)
   const R t = v_k - hi;
   bool constant = (k == row.size());
   if (!constant) {
-    R nxt;
+    R nxt = -num<R>::inf();
     Taken<R> peek = tk;
     take_next<R>(row, peek, nxt);
     constant = (t >= nxt - eps);
@@ -446,7 +447,7 @@ SDCAB_D void row_max_sumexp(const Row& row, Pred in, R& mx, R& s, int& count) {
     R x = static_cast<R>(xd);
     if (in(x, i)) {
       ++c;
-      if (bi == INT_MAX || x > best) { best = x; bi = i; }
+      if (x > best || (bi == INT_MAX && x == x)) { best = x; bi = i; }   // NaN as in take_next
     }
   });
 #if defined(SDCAB_WARP_GROUP)
@@ -525,7 +526,7 @@ SDCAB_D Thr<R> thr_topk_entropy(const Row& row, int k) {
   int num_U = 0;
   R cur_max = mx;  // maximum of the entries not in U
   for (num_U = 1; num_U < k; ++num_U) {
-    R v;
+    R v = -num<R>::inf();
     take_next<R>(row, tk, v);  // v == cur_max
     min_U = v; sum_U += v; k_u -= 1;
     row_max_sumexp<R>(row, [&](R x, int i) { return !tk.has(x, i); }, cur_max, z, cnt);
@@ -911,14 +912,14 @@ SDCAB_D Thr<R> thr_topk_entropy_biased(const Row& row, int k, R alpha, bool outp
   // the two-dimensional KKT system in (s, t) by Newton steps   (:72-175)
   const R log_k = log_(K), log_alpha = log_(alpha);
   Taken<R> tk;
-  R v;
+  R v = -num<R>::inf();
   take_next<R>(row, tk, v);
   R min_U = v, sum_U = v;
   int num_U = 1;
   const R eps16 = 16 * num<R>::eps();
   for (; num_U < m;) {
     Taken<R> nx = tk;
-    R cur;
+    R cur = -num<R>::inf();
     take_next<R>(row, nx, cur);  // largest entry outside U
     const R U = static_cast<R>(num_U);
     s = R(0.999); t = cur;

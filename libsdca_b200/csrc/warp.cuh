@@ -79,9 +79,14 @@ SDCAB_D int warp_sum(int v) {
 #endif
 }
 
+// Maxima and minima leave NaN out (a group of nothing else gives the infinity of an empty one).  A
+// comparison with NaN is false from either side: the two lanes of an exchange would keep different
+// values, and lanes that disagree take different ways through loops with reductions in them, where they
+// would wait for one another for ever.
 template <typename T>
 SDCAB_D T warp_max(T v) {
 #if defined(SDCAB_WARP_GROUP)
+  v = (v == v) ? v : static_cast<T>(-INFINITY);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     T w = __shfl_xor_sync(kFullMask, v, o);
@@ -94,6 +99,7 @@ SDCAB_D T warp_max(T v) {
 template <typename T>
 SDCAB_D T warp_min(T v) {
 #if defined(SDCAB_WARP_GROUP)
+  v = (v == v) ? v : static_cast<T>(INFINITY);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     T w = __shfl_xor_sync(kFullMask, v, o);
@@ -101,21 +107,6 @@ SDCAB_D T warp_min(T v) {
   }
 #endif
   return v;
-}
-
-// Largest value together with the smallest index that holds it.
-template <typename T>
-SDCAB_D void warp_argmax(T& v, int& idx) {
-#if defined(SDCAB_WARP_GROUP)
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    T w = __shfl_xor_sync(kFullMask, v, o);
-    int j = __shfl_xor_sync(kFullMask, idx, o);
-    if (w > v || (w == v && j < idx)) { v = w; idx = j; }
-  }
-#else
-  (void)v; (void)idx;
-#endif
 }
 
 // ---- numeric traits --------------------------------------------------------
