@@ -71,15 +71,18 @@ eval_softmax_loss_kernel(LossArgs g, const Data* __restrict__ scores, const Data
     own = __shfl_sync(kFullMask, own, y & 31);
     top = largest_of_lanes(top);
     // the other classes scoring at least as high as the label (eval/primal.h:42-52), the sum of
-    // exp(s_j - top) without one instance of the largest score
+    // exp(s_j - top) without one instance of the largest score.  The entries past the row's end, -inf,
+    // are left out of all three: a label's score of -inf is no higher than they are.
     int rank = 0, ties = 0;
     R sum = 0;
 #pragma unroll
     for (int i = 0; i < NE; ++i) {
       const int j = lane + 32 * i;
-      rank += (j != y && s[i] >= own) ? 1 : 0;
-      if (s[i] == top) ++ties;
-      else if (j < m) sum += exp_(static_cast<R>(s[i]) - static_cast<R>(top));
+      if (j < m) {
+        rank += (j != y && s[i] >= own) ? 1 : 0;
+        if (s[i] == top) ++ties;
+        else sum += exp_(static_cast<R>(s[i]) - static_cast<R>(top));
+      }
     }
     sum += static_cast<R>(ties);
     sum = warp_sum(sum) - R(1);

@@ -69,3 +69,58 @@ def test_softmax_loss_of_many_examples_repeats_bit_for_bit(cuda_lib):
     top = scores.max(axis=1)
     exact = (top + np.log(np.exp(scores - top[:, None]).sum(axis=1)) - scores[np.arange(len(X)), labels]).sum()
     assert abs(first["primal_loss"] - exact) <= 1e-12 * abs(exact)
+
+
+def guarded_sums(mod, X, labels, W, dtype, precision):
+    """One evaluation in a workspace of exactly the required size with a pattern behind it: the sums, and
+    whether the pattern is still there."""
+    import ctypes as C
+
+    import torch
+    from libsdca_b200 import binding as b
+    m = W.shape[0]
+    obj = b.make_objective(0, precision=precision)
+    problem = b.make_problem(X, labels, W=W, is_train=False)
+    suffix = "f32" if dtype == np.float32 else "f64"
+    query = mod.lib()["sdcab_eval_workspace_bytes"]
+    query.restype = C.c_size_t
+    need = query(C.c_int64(X.shape[0]), C.c_int64(m), C.c_int64(np.dtype(dtype).itemsize))
+    guard = 16384
+    work = torch.full((need + guard,), 0x5a, dtype=torch.uint8, device="cuda")
+    sums = torch.zeros(8 + m, dtype=torch.float64, device="cuda")
+    b.eval_sums_(obj, problem, sums, suffix, work, need)
+    return sums.cpu().numpy(), bool((work[need:] == 0x5a).all())
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("precision", ["double", "float"])
+def test_softmax_loss_of_infinite_scores(cuda_lib, dtype, precision):
+    """A label's score of -inf, and rows of infinities: the ranks are those of the general kernel, and
+    nothing is written past the histogram."""
+    from libsdca_b200 import binding as b
+    rng = np.random.default_rng(stable_seed("infinite", str(dtype), precision))
+    for m in (2, 20, 32, 101, 128, 200, 256, 257, 300, 600, 1000, 1024):
+        n = 12
+        scores = rng.standard_normal((m, n))
+        labels = rng.integers(0, m, n)
+        scores[labels[0], 0] = -np.inf
+        scores[labels[1], 1] = scores[(labels[1] + 1) % m, 1] = -np.inf
+        scores[:, 2] = -np.inf
+        scores[labels[3], 3] = np.inf
+        scores[(labels[4] + 1) % m, 4] = np.inf
+        scores[:, 5] = np.inf
+        scores[labels[6], 6] = np.nan
+        scores[(labels[7] + 1) % m, 7] = np.nan
+        # one feature and one example at a time: in a product of several, 0 * inf would reach other scores
+        for e in range(n):
+            W = dev(scores[:, e:e + 1].astype(dtype))
+            args = (cuda_lib, dev(np.ones((1, 1), dtype=dtype)), dev(labels[e:e + 1]), W, dtype, precision)
+            got, kept = guarded_sums(*args)
+            try:
+                b.test_set("loss_general", 1)
+                general, _ = guarded_sums(*args)
+            finally:
+                b.test_set("loss_general", 0)
+            assert kept, (m, e)
+            assert np.array_equal(got[8:], general[8:]) and got[8:].sum() == 1, (m, e)
+            assert got[6] == 0, (m, e)
