@@ -84,9 +84,12 @@ eval_softmax_loss_kernel(LossArgs g, const Data* __restrict__ scores, const Data
         else sum += exp_(static_cast<R>(s[i]) - static_cast<R>(top));
       }
     }
-    sum += static_cast<R>(ties);
-    sum = warp_sum(sum) - R(1);
-    rank = warp_sum(rank);
+    sum = warp_sum(sum);
+    const int counts = warp_sum((ties << 16) + rank);
+    rank = counts & 0xffff; ties = counts >> 16;
+    // The one that is left out never enters the sum: next to it a small remainder would be lost.  Every
+    // other tie adds exp(0) (and makes the loss of several infinite scores NaN, as the general kernel's).
+    if (ties != 1) sum += static_cast<R>(ties - 1) * exp_(static_cast<R>(top) - static_cast<R>(top));
     if (lane == 0) {
       if (rank < kHistLocal) atomicAdd(&local_hist[rank], 1u);
       else atomicAdd(&hist[rank], 1ull);

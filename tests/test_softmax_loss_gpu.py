@@ -95,8 +95,8 @@ def guarded_sums(mod, X, labels, W, dtype, precision):
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("precision", ["double", "float"])
 def test_softmax_loss_of_infinite_scores(cuda_lib, dtype, precision):
-    """A label's score of -inf, and rows of infinities: the ranks are those of the general kernel, and
-    nothing is written past the histogram."""
+    """A label's score of -inf, and rows of infinities: the ranks and the loss are those of the general kernel,
+    and nothing is written past the histogram."""
     from libsdca_b200 import binding as b
     rng = np.random.default_rng(stable_seed("infinite", str(dtype), precision))
     for m in (2, 20, 32, 101, 128, 200, 256, 257, 300, 600, 1000, 1024):
@@ -124,3 +124,23 @@ def test_softmax_loss_of_infinite_scores(cuda_lib, dtype, precision):
             assert kept, (m, e)
             assert np.array_equal(got[8:], general[8:]) and got[8:].sum() == 1, (m, e)
             assert got[6] == 0, (m, e)
+            assert np.allclose(got[0], general[0], rtol=1e-5 if "float" in (precision, np.dtype(dtype).name[:5]) else 1e-12,
+                               equal_nan=True), (m, e, got[0], general[0])
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("precision", ["double", "float"])
+def test_softmax_loss_of_confident_models(cuda_lib, dtype, precision):
+    """Losses far below one: what is left of an example's loss is the small sum next to the one of its
+    own class."""
+    rng = np.random.default_rng(stable_seed("confident", str(dtype), precision))
+    for m, margin in ((2, 40.0), (31, 25.0), (101, 20.0), (129, 30.0), (300, 12.0), (1000, 20.0)):
+        W = (-margin - rng.uniform(0, 2, (m, 1))).astype(dtype)
+        W[m // 2] = 0
+        labels = np.full(50, m // 2)
+        got = cuda_lib.evaluate(0, dev(np.ones((50, 1), dtype=dtype)), dev(labels), W=dev(W), is_train=False,
+                                precision=precision)
+        loss = 50 * np.log1p(np.exp(np.delete(W, m // 2).astype(np.float64)).sum())
+        # m exponentials, 4 eps each, and their sum in another order
+        eps = np.finfo(np.float32 if dtype == np.float32 or precision == "float" else np.float64).eps
+        assert abs(got["primal_loss"] / loss - 1) <= 16 * eps + 1e-14, (m, margin)
