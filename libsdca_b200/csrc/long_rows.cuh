@@ -188,17 +188,24 @@ __device__ __forceinline__ void block_sort_desc(Data* v, int count) {
 // The thresholds from the `total` candidates in `slots`, by warp 0.  `s` is the sum that pass 1
 // took: of the positive entries (cone), of the entries clipped to [0, hi] (knapsack_le).
 template <typename R, int PROX, typename Data>
-__device__ __forceinline__ FastStatus long_row_solve(const Data* slots, int total, int m, R s,
+__device__ __forceinline__ FastStatus long_row_solve(Data* slots, int total, int m, R s,
                                                      const ProxParams& q, const TopkConsts<R>& tc, R rho,
                                                      R* sorted, int lane, Thr<R>& thr) {
   const R rhs = static_cast<R>(q.rhs);
   if (!LongKind<PROX>::kKnapsack && total <= q.k) return kFastNeedsFullRow;
   if (total < 1) return kFastNeedsFullRow;
-  StridedRow<Data> list(slots, total);
+  // Slots are handed out in the order in which the block's threads come by.  Lists that one warp holds
+  // are sorted here, longer ones by the block: every sum over them is the same from run to run.
   LaneRow<Data> cand;
   cand.valid = lane < total;
   cand.x = lane < total ? slots[lane] : -num<Data>::inf();
   cand.reported = m;
+  if (LongKind<PROX>::kKnapsack && total <= 32) {
+    cand.x = warp_sort_desc(cand.x, lane);
+    if (cand.valid) slots[lane] = cand.x;
+    __syncwarp();
+  }
+  StridedRow<Data> list(slots, total);
   if (LongKind<PROX>::kSimplex) {
     if (total <= 32)
       return topk_simplex_of_candidates<R>(cand, total, m, q.k, rhs, rho, tc, sorted, lane, thr);
@@ -317,8 +324,6 @@ long_rows_kernel(const Data* a, Data* out, int m, long long n, ProxParams q, int
       __syncthreads();
       const int total = s_count;
       if (total > 32 && total <= kLongSlots) {
-        // the slots were handed out in no particular order: sorted, every sum over them is the
-        // same from run to run
         int pow2 = 64;
         while (pow2 < total) pow2 <<= 1;
         for (int i = total + tid; i < pow2; i += blockDim.x) slots[i] = -num<Data>::inf();

@@ -91,27 +91,32 @@ def test_long_rows(oracle, cuda_lib, name, dtype, precision):
 
 
 @pytest.mark.parametrize("name", LONG)
-def test_long_rows_with_crowded_tops(oracle, cuda_lib, name):
-    """More candidates than one warp takes, than the block keeps, all entries equal, no finite
-    row, one dominating entry: the same answers as the general routine gives."""
+@pytest.mark.parametrize("dtype,m", [(np.float64, 1000), (np.float32, 3000)])
+def test_long_rows_with_crowded_tops(oracle, cuda_lib, name, dtype, m):
+    """More candidates than one warp takes, than the block keeps, all entries equal, one dominating
+    entry: the same answers as the general routine gives."""
     rng = np.random.default_rng(stable_seed("crowded", name))
-    m = 3000
     rows = [1e-3 * rng.standard_normal(m), 1e-2 * rng.standard_normal(m), 0.1 * rng.standard_normal(m),
             np.full(m, 0.25), np.full(m, -1.0), np.zeros(m), rng.standard_normal(m)]
     rows[6][17] = 50.0
-    a = np.stack(rows)
+    a = np.stack(rows).astype(dtype)
     for kw in (dict(), dict(rhs=4.0)) if name != "topk_cone" else (dict(),):
         k = dict(k=5) if name.startswith("topk") else {}
         check(oracle, cuda_lib, name, a, "double", **kw, **k)
-        check(oracle, cuda_lib, name, a.astype(np.float32), "double", **kw, **k)
 
 
-def test_long_rows_repeat_bit_for_bit(cuda_lib):
+@pytest.mark.parametrize("name", LONG)
+@pytest.mark.parametrize("dtype,m", [(np.float64, 513), (np.float64, 1024), (np.float32, 1025), (np.float32, 5000)])
+def test_long_rows_repeat_bit_for_bit(cuda_lib, name, dtype, m):
+    """Few candidates and many: the order in which a block's threads find them must not show."""
+    import torch
     rng = np.random.default_rng(8)
-    a = 0.05 * rng.standard_normal((300, 5000))
-    for name in LONG:
-        first = run_dev(cuda_lib, name, a, 0)
-        assert np.array_equal(first, run_dev(cuda_lib, name, a, 0)), name
+    for scale in (1.0, 0.05):
+        a = torch.from_numpy((scale * rng.standard_normal((4000, m))).astype(dtype)).cuda()
+        kw = dict(k=5) if name.startswith("topk") else {}
+        first = cuda_lib.prox(a, name, **kw)
+        for _ in range(6):
+            assert torch.equal(first, cuda_lib.prox(a, name, **kw)), (name, m, scale)
 
 
 @pytest.mark.parametrize("name", ["knapsack_eq", "knapsack_le", "knapsack_le_biased", "topk_simplex",
