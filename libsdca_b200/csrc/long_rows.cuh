@@ -209,23 +209,7 @@ __device__ __forceinline__ FastStatus long_row_solve(Data* slots, int total, int
   if (LongKind<PROX>::kSimplex) {
     if (total <= 32)
       return topk_simplex_of_candidates<R>(cand, total, m, q.k, rhs, rho, tc, sorted, lane, thr);
-    // thr_topk_simplex without its last resort, which needs the whole row
-    const R eps = tc.eps_rhs;
-    const Projection proj = topk_special_cases<R>(list, q.k, tc.K + tc.rho_k2, thr);
-    if (proj == kProjZero) return kFastDone;
-    if (proj == kProjConstant && !(tc.K * thr.hi > rhs + eps)) return kFastDone;
-    thr = thr_knapsack_eq<R>(list, R(0), tc.H, rhs);
-    if (proj == kProjConstant) return kFastDone;
-    bool lt;
-    if (thr.nU == 0) {
-      lt = thr.t < rho * rhs - eps;
-    } else {
-      int cnt; R sum_U;
-      row_count_sum_gt<R>(list, thr.cutU, cnt, sum_U);
-      const R num_U = static_cast<R>(cnt);
-      lt = tc.K * (sum_U + (tc.K - num_U) * thr.t) < rhs * (num_U + tc.rho_k2) - eps;
-    }
-    return lt ? kFastNeedsFullRow : kFastDone;
+    return topk_simplex_without_search<R>(list, q.k, rhs, rho, false, thr) ? kFastDone : kFastNeedsFullRow;
   }
   if (LongKind<PROX>::kCone) {
     R top;

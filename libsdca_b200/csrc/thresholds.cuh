@@ -407,31 +407,32 @@ SDCAB_D Thr<R> thr_topk_cone(const Row& row, int k, R rho) {
 }
 
 // min 0.5(<x,x> + rho<1,x>^2) - <a,x>,  <1,x> <= rhs,  0 <= x_i <= <1,x>/k
-// (include/sdca/prox/topk_simplex.h:9-68, topk_simplex_biased.h:9-71)
+// (include/sdca/prox/topk_simplex.h:9-68, topk_simplex_biased.h:9-71), as far as it needs no more than
+// the support and the k + 1 largest entries; false where the cone's search has to decide.
 template <typename R, typename Row>
-SDCAB_D Thr<R> thr_topk_simplex(const Row& row, int k, R rhs, R rho, bool accurate = false) {
+SDCAB_D bool topk_simplex_without_search(const Row& row, int k, R rhs, R rho, bool accurate, Thr<R>& thr) {
   const R K = static_cast<R>(k), lo = 0;
   const R eps = num<R>::eps() * max_(R(1), abs_(rhs));
   const R rho_k2 = rho * K * K;
-  Thr<R> thr;
   const Projection proj = topk_special_cases<R>(row, k, K + rho_k2, thr);
-  if (proj == kProjZero) return thr;
+  if (proj == kProjZero) return true;
   if (proj == kProjConstant) {
-    if (K * thr.hi > rhs + eps) return thr_knapsack_eq<R>(row, lo, rhs / K, rhs, accurate);
-    return thr;
+    if (K * thr.hi > rhs + eps) thr = thr_knapsack_eq<R>(row, lo, rhs / K, rhs, accurate);
+    return true;
   }
-  Thr<R> eq = thr_knapsack_eq<R>(row, lo, rhs / K, rhs, accurate);
-  bool lt;
-  if (eq.nU == 0) {
-    lt = eq.t < rho * rhs - eps;
-  } else {
-    int cnt; R sum_U;
-    row_count_sum_gt<R>(row, eq.cutU, cnt, sum_U);
-    const R num_U = static_cast<R>(cnt);
-    lt = K * (sum_U + (K - num_U) * eq.t) < rhs * (num_U + rho_k2) - eps;
-  }
-  if (lt) return thr_topk_cone_search<R>(row, k, rho);
-  return eq;
+  thr = thr_knapsack_eq<R>(row, lo, rhs / K, rhs, accurate);
+  if (thr.nU == 0) return !(thr.t < rho * rhs - eps);
+  int cnt; R sum_U;
+  row_count_sum_gt<R>(row, thr.cutU, cnt, sum_U);
+  const R num_U = static_cast<R>(cnt);
+  return !(K * (sum_U + (K - num_U) * thr.t) < rhs * (num_U + rho_k2) - eps);
+}
+
+template <typename R, typename Row>
+SDCAB_D Thr<R> thr_topk_simplex(const Row& row, int k, R rhs, R rho, bool accurate = false) {
+  Thr<R> thr;
+  if (topk_simplex_without_search<R>(row, k, rhs, rho, accurate, thr)) return thr;
+  return thr_topk_cone_search<R>(row, k, rho);
 }
 
 // ---- entropic projections ---------------------------------------------------

@@ -103,3 +103,41 @@ def test_evaluation_of_scores_that_are_nan(cuda_lib, objective, dtype):
                 # no class scores at least as high as NaN: the example counts as rank 0
                 want = (rest["accuracy"] * (n - 1) + 1) / n
                 assert np.abs(got["accuracy"] - want).max() <= 1e-9, (n, m)
+
+
+# Rows of which a part is ruled out by a very small value.  The answer is the projection of the other
+# entries and 0 for these: the operators' supports lie near the top of a row.
+MASKED = {"knapsack_eq": {}, "knapsack_le": {}, "knapsack_le_biased": dict(rho=0.1), "topk_simplex": dict(k=3),
+          "topk_simplex_biased": dict(k=3, rho=0.01), "topk_cone": dict(k=3), "entropy": {}, "topk_entropy": dict(k=3)}
+
+
+@pytest.mark.parametrize("name", MASKED)
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_masked_entries(oracle, cuda_lib, name, dtype):
+    import torch
+    rng = np.random.default_rng(stable_seed("masked", name, str(dtype)))
+    lowest = float(np.finfo(dtype).min)
+    # one thread per row (on and off the vector grid), registers (on and off), a block per row
+    for m, n, offset, values in ((10, 30000, 0, (-np.inf, lowest, -1e30)), (31, 93000, 1, (-np.inf, lowest, -1e30)),
+                                 (32, 96000, 0, (-np.inf, lowest, -1e30)), (40, 120000, 0, (-np.inf, lowest, -1e30)),
+                                 (100, 60, 0, (-np.inf, lowest, -1e30)), (101, 60, 0, (-np.inf, lowest, -1e30)),
+                                 (300, 60, 1, (-np.inf, lowest, -1e30)), (1000, 60, 0, (lowest, -1e30)),
+                                 (1025, 60, 0, (lowest, -1e30))):
+        if m == 1025 and dtype == np.float64:
+            continue                     # rows of doubles this long are the general kernel's
+        for value in values:
+            rows, kept = 60, m - max(3, m // 3)
+            a = rng.standard_normal((rows, m)).astype(dtype) + 1
+            where = rng.permuted(np.tile(np.arange(m), (rows, 1)), axis=1)
+            keep, drop = np.sort(where[:, :kept], axis=1), where[:, kept:]
+            part = np.take_along_axis(a, keep, axis=1)
+            np.put_along_axis(a, drop, dtype(value), axis=1)
+            flat = torch.empty(n * m + 4, dtype=torch.from_numpy(a).dtype, device="cuda")
+            t = flat[offset:offset + n * m].view(n, m)
+            t.copy_(torch.from_numpy(a).cuda()[torch.arange(n, device="cuda") % rows])
+            cuda_lib.prox_(t, name, **MASKED[name])
+            x = t[:rows].cpu().numpy()
+            assert rows_repeat(t, rows, tolerance(dtype, "double", m)), (name, m, value)
+            assert not np.take_along_axis(x, drop, axis=1).any(), (name, m, value)
+            err = scaled_error(np.take_along_axis(x, keep, axis=1), oracle.prox(name, part, **MASKED[name]), part).max()
+            assert err <= tolerance(dtype, "double", m), (name, m, value, err)
