@@ -37,6 +37,21 @@ int get_device_info(DeviceInfo* out) {
   return SDCAB_OK;
 }
 
+static std::mutex g_shared_limit_mutex;
+
+int allow_shared_memory(const void* kernel, size_t bytes) {
+  auto get = [&]() -> size_t {
+    cudaFuncAttributes attr;
+    if (cudaFuncGetAttributes(&attr, kernel) != cudaSuccess) return 0;   // so will the setting
+    return static_cast<size_t>(attr.maxDynamicSharedSizeBytes);
+  };
+  auto set = [&](size_t want) -> int {
+    SDCAB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(want)));
+    return SDCAB_OK;
+  };
+  return raise_limit(g_shared_limit_mutex, bytes, get, set);
+}
+
 static const int kSlots = 8;
 static Workspace g_ws[kMaxDevices][kSlots];
 

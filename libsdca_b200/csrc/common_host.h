@@ -30,6 +30,10 @@ struct DeviceInfo {
 };
 int get_device_info(DeviceInfo* info);
 
+// Allows `kernel` that much dynamic shared memory for a launch.  The limit belongs to the kernel on its
+// device, not to the launch, and is only ever raised.
+int allow_shared_memory(const void* kernel, size_t bytes);
+
 // Grow-only per-device scratch owned by the library; used only by the
 // host-buffer entry points (the *_dev entry points allocate nothing unless
 // their documentation says so).  The table is guarded by a mutex, and the

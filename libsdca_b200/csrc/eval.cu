@@ -384,8 +384,8 @@ int eval_sums_dev(const sdcab_objective* obj, const sdcab_problem* p, double* su
   auto kd = eval_loss_kernel<Data, double>;
   auto kf = eval_loss_kernel<Data, float>;
   if (smem > 48 * 1024) {
-    SDCAB_CUDA_TRY(cudaFuncSetAttribute(kd, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    SDCAB_CUDA_TRY(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    rc = allow_shared_memory(fl ? reinterpret_cast<const void*>(kf) : reinterpret_cast<const void*>(kd), smem);
+    if (rc) return rc;
   }
   for (long long first = 0; first < n; first += L.chunk) {
     const long long count = std::min(L.chunk, n - first);
@@ -653,8 +653,8 @@ int eval_sums_fixed_scratch(const sdcab_objective* obj, const sdcab_problem* p, 
   auto kd = eval_loss_kernel<Data, double>;
   auto kf = eval_loss_kernel<Data, float>;
   if (smem > 48 * 1024) {
-    SDCAB_CUDA_TRY(cudaFuncSetAttribute(kd, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    SDCAB_CUDA_TRY(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    rc = allow_shared_memory(fl ? reinterpret_cast<const void*>(kf) : reinterpret_cast<const void*>(kd), smem);
+    if (rc) return rc;
   }
   for (long long first = 0; first < n; first += chunk) {
     const long long count = std::min(chunk, n - first);

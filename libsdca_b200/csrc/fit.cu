@@ -246,9 +246,8 @@ struct BlockRunner {
     chain_smem = s_on_chip ? with_s : fixed;
     if (chain_smem + 2048 > info.smem_optin) return SDCAB_ERR_TOO_LARGE;
     chain = pick_chain_kernel<Data, R>(o, m, s_on_chip != 0);
-    SDCAB_CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(chain.kernel),
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(chain_smem)));
+    int rc = allow_shared_memory(reinterpret_cast<const void*>(chain.kernel), chain_smem);
+    if (rc) return rc;
     const bool kernel_input = t->input_kind == SDCAB_INPUT_KERNEL;
     const size_t n = static_cast<size_t>(t->n), block_row = static_cast<size_t>(kBlockSteps) * m,
                  block_block = static_cast<size_t>(kBlockSteps) * kBlockSteps;
@@ -260,7 +259,7 @@ struct BlockRunner {
     bytes += kernel_input ? DeviceBuffers::padded(n * sizeof(int))
                           : 2 * DeviceBuffers::padded(block_row * sizeof(Data)) +
                                 DeviceBuffers::padded(g_slices * 2 * block_block * sizeof(Data));
-    int rc = buf.reserve(bytes); if (rc) return rc;
+    rc = buf.reserve(bytes); if (rc) return rc;
     rc = buf.alloc(&order, n); if (rc) return rc;
     for (int h = 0; h < 2; ++h) {
       rc = buf.alloc(&s_parts[h], static_cast<size_t>(slices) * kBlockSteps * m); if (rc) return rc;

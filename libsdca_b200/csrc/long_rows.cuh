@@ -347,9 +347,10 @@ int launch_long(const Data* a, Data* out, int m, long long n, const ProxParams& 
   // Short rows want many small blocks (a block's barriers and its one solving warp are covered by
   // the others), rows that leave room for one or two copies on an SM want as many threads as fit.
   const int threads = row_bytes <= 16 * 1024 ? 128 : (row_bytes <= 56 * 1024 ? 256 : kLongMaxThreads);
-  if (smem > 32 * 1024)
-    SDCAB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(smem)));
+  if (smem > 32 * 1024) {
+    rc = allow_shared_memory(reinterpret_cast<const void*>(kernel), smem);
+    if (rc) return rc;
+  }
   int per_sm = 0;
   SDCAB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
   if (per_sm < 1) per_sm = 1;

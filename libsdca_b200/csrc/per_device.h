@@ -4,6 +4,9 @@
 // several GPUs.  Plain C++, so the CPU tests can use it directly.
 #pragma once
 
+#include <cstddef>
+#include <mutex>
+
 namespace sdcab {
 
 constexpr int kMaxDevices = 64;
@@ -25,5 +28,14 @@ struct OncePerDevice {
     return true;
   }
 };
+
+// Raises a limit that calls of several host threads share (`get` reads it, `set` writes it and returns
+// a status): never lowered, so that what one thread has asked for still holds when it makes use of it,
+// whatever smaller amount another thread asks for in between.
+template <typename Get, typename Set>
+int raise_limit(std::mutex& guard, size_t want, Get&& get, Set&& set) {
+  std::lock_guard<std::mutex> lock(guard);
+  return get() >= want ? 0 : set(want);
+}
 
 }  // namespace sdcab

@@ -135,8 +135,8 @@ int launch_rows(const Data* a, Data* out, int m, long long n, const ProxParams& 
   const size_t room = kUneven ? info.smem_optin / 18 : info.smem_optin;
   if (smem > room) { staged = 0; smem = 0; }
   if (smem > 48 * 1024) {
-    SDCAB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(smem)));
+    rc = allow_shared_memory(reinterpret_cast<const void*>(kernel), smem);
+    if (rc) return rc;
   }
   long long most = 0x7fffffffLL;
   if (!kUneven) {
@@ -177,9 +177,10 @@ int launch_two_simplex_sort(const Data* a, Data* out, int m, long long n, const 
   auto kernel = two_simplex_sort_kernel<Data, R>;
   // the kernel also has about 1 KB of static shared memory, which counts towards the 48 KB
   // that need no opt-in
-  if (smem + 2048 > 48 * 1024)
-    SDCAB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(smem)));
+  if (smem + 2048 > 48 * 1024) {
+    rc = allow_shared_memory(reinterpret_cast<const void*>(kernel), smem);
+    if (rc) return rc;
+  }
   const long long want = (n + warps - 1) / warps;
   const int blocks = static_cast<int>(std::max<long long>(1, std::min<long long>(want, 8LL * info.sm_count)));
   kernel<<<blocks, kSortThreads, smem, stream>>>(a, out, m, n, q, thr_out, apply, pa, pb);

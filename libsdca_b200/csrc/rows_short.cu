@@ -171,9 +171,10 @@ int launch_short(const Data* a, Data* out, int m, long long n, const ProxParams&
   auto kernel = short_rows_kernel<Data, PROX>;
   const int pitch = m | 1;
   const size_t smem = static_cast<size_t>(kShortThreads) * pitch * sizeof(Data);
-  if (smem > 48 * 1024)
-    SDCAB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(smem)));
+  if (smem > 48 * 1024) {
+    rc = allow_shared_memory(reinterpret_cast<const void*>(kernel), smem);
+    if (rc) return rc;
+  }
   int per_sm = 0;
   SDCAB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kShortThreads, smem));
   const long long want = (n + kShortThreads - 1) / kShortThreads;

@@ -15,7 +15,7 @@ def build():
         os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
     if os.path.exists(SO) and all(os.path.getmtime(d) <= os.path.getmtime(SO) for d in deps):
         return SO
-    subprocess.run(["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-x", "c++",
+    subprocess.run(["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-pthread", "-x", "c++",
                     os.path.join(HERE, "hostsim.cpp"), "-o", SO], check=True)
     return SO
 

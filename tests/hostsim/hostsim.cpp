@@ -320,3 +320,26 @@ extern "C" uint64_t sdcab_hostsim_once_per_device(const int* order, int count) {
     if (once.first_time(order[i])) bits |= uint64_t(1) << i;
   return bits;
 }
+
+// Threads that ask for different amounts of a limit they share, the way launches ask for dynamic shared
+// memory: the number of times that the amount did not hold when a thread came to use it.
+#include <atomic>
+#include <thread>
+
+extern "C" int64_t sdcab_hostsim_raise_limit(int threads, int rounds) {
+  std::atomic<size_t> limit{0};
+  std::atomic<int64_t> failed{0};
+  std::mutex guard;
+  std::vector<std::thread> pool;
+  for (int t = 0; t < threads; ++t)
+    pool.emplace_back([&, t] {
+      const size_t want = 1000 + 100 * static_cast<size_t>(t);
+      for (int r = 0; r < rounds; ++r) {
+        sdcab::raise_limit(guard, want, [&] { return limit.load(); }, [&](size_t v) { limit = v; return 0; });
+        std::this_thread::yield();
+        if (limit < want) ++failed;
+      }
+    });
+  for (std::thread& t : pool) t.join();
+  return failed;
+}

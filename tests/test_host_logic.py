@@ -143,3 +143,11 @@ def test_test_switches_are_named():
     assert lib.sdcab_test_set(b"eval_chunk", C.c_int64(0)) == 0
     assert lib.sdcab_test_set(b"gemm_simt", C.c_int64(0)) == 0
     assert lib.sdcab_test_set(b"no_such_switch", C.c_int64(1)) == -1
+
+
+def test_a_shared_limit_is_never_lowered(hostsim):
+    """Calls of several host threads whose launches need different amounts of shared memory: what a
+    thread has asked for holds when it launches."""
+    f = hostsim.lib.sdcab_hostsim_raise_limit
+    f.restype = C.c_int64
+    assert f(C.c_int(4), C.c_int(20000)) == 0
