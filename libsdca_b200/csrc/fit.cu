@@ -242,10 +242,15 @@ struct BlockRunner {
     const size_t fixed = (kBlockSteps * kBlockSteps + 2 * m) * sizeof(double) + 5 * m * sizeof(Data) +
                          static_cast<size_t>(2 * ((m + 31) / 32) + 2) * sizeof(unsigned);
     const size_t with_s = fixed + static_cast<size_t>(kBlockSteps) * m * sizeof(double);
-    s_on_chip = (with_s + 2048 <= info.smem_optin) ? 1 : 0;
-    chain_smem = s_on_chip ? with_s : fixed;
-    if (chain_smem + 2048 > info.smem_optin) return SDCAB_ERR_TOO_LARGE;
-    chain = pick_chain_kernel<Data, R>(o, m, s_on_chip != 0);
+    // beside the kernel's own static shared memory (up to 4 KB, by its step)
+    cudaFuncAttributes attr;
+    for (s_on_chip = 1; s_on_chip >= 0; --s_on_chip) {
+      chain = pick_chain_kernel<Data, R>(o, m, s_on_chip != 0);
+      chain_smem = s_on_chip ? with_s : fixed;
+      SDCAB_CUDA_TRY(cudaFuncGetAttributes(&attr, reinterpret_cast<const void*>(chain.kernel)));
+      if (chain_smem + attr.sharedSizeBytes <= info.smem_optin) break;
+    }
+    if (s_on_chip < 0) return SDCAB_ERR_TOO_LARGE;
     int rc = allow_shared_memory(reinterpret_cast<const void*>(chain.kernel), chain_smem);
     if (rc) return rc;
     const bool kernel_input = t->input_kind == SDCAB_INPUT_KERNEL;

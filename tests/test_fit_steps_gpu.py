@@ -102,3 +102,27 @@ def test_multilabel_hinge_steps(oracle, cuda_lib, objective, dtype, kernel):
         g = cuda_lib.fit_(IDS[objective], dev(data), dev(labels), A, W=W, kernel=kernel, offsets=dev(offsets), **kw)
         compare(r, g, A_ref, W_ref, A.cpu().numpy(), None if kernel else W.cpu().numpy(),
                 1e-9 if dtype == np.float64 else 2e-4, (n, m, c, kernel))
+
+
+@pytest.mark.parametrize("objective", ["l2_topk_hinge", "l2_hinge_topk", "l2_entropy"])
+@pytest.mark.parametrize("dtype,classes", [(np.float64, range(342, 350)), (np.float32, range(354, 362))])
+def test_class_counts_at_which_the_score_rows_leave_shared_memory(oracle, cuda_lib, objective, dtype, classes):
+    for m in classes:
+        check_kernel(oracle, cuda_lib, objective, dtype, 70, m, 3 if "topk" in objective else 1, 1)
+
+
+def test_class_counts_beyond_shared_memory_are_refused(cuda_lib):
+    """Even one score row has to fit: up to there a fit runs, from there on it says so."""
+    import torch
+    refused = []
+    for m in (3400, 3475, 3485, 3500, 3512, 3520, 3600):
+        K = torch.eye(4, dtype=torch.float64, device="cuda")
+        A = torch.zeros(4, m, dtype=torch.float64, device="cuda")
+        try:
+            cuda_lib.fit_("msvm", K, torch.arange(4, device="cuda"), A, kernel=True, max_epoch=1, eval_epoch=1)
+            refused.append(False)
+            assert bool((A.sum(dim=1).abs() < 1e-12).all()) and bool(A.any())
+        except cuda_lib.SdcabError as error:
+            assert "too_large" in str(error), error
+            refused.append(True)
+    assert refused == sorted(refused) and not refused[0] and refused[-1]
