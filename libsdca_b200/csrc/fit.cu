@@ -154,13 +154,12 @@ template <> int eval_sums_call<double>(const sdcab_objective* o, const sdcab_pro
 }
 
 struct DeviceBuffers {
-  void* p[24] = {nullptr};
-  int count = 0;
+  std::vector<void*> owned;     // three for each held-out set, and there may be any number of those
   cudaStream_t stream = nullptr, ahead = nullptr;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   cudaEvent_t ev_product[2] = {nullptr, nullptr}, ev_steps[2] = {nullptr, nullptr}, ev_start = nullptr;
   ~DeviceBuffers() {
-    for (int i = 0; i < count; ++i) cudaFree(p[i]);
+    for (void* ptr : owned) cudaFree(ptr);
     for (int i = 0; i < 4; ++i) if (ev[i]) cudaEventDestroy(ev[i]);
     for (int i = 0; i < 2; ++i) {
       if (ev_product[i]) cudaEventDestroy(ev_product[i]);
@@ -178,7 +177,7 @@ struct DeviceBuffers {
   int reserve(size_t bytes) {
     void* ptr = nullptr;
     SDCAB_CUDA_TRY(cudaMalloc(&ptr, bytes));
-    p[count++] = ptr;
+    owned.push_back(ptr);
     arena = static_cast<unsigned char*>(ptr);
     arena_bytes = bytes;
     return SDCAB_OK;
@@ -193,7 +192,7 @@ struct DeviceBuffers {
     }
     void* ptr = nullptr;
     SDCAB_CUDA_TRY(cudaMalloc(&ptr, bytes));
-    p[count++] = ptr;
+    owned.push_back(ptr);
     *out = static_cast<T*>(ptr);
     return SDCAB_OK;
   }

@@ -126,3 +126,22 @@ def test_class_counts_beyond_shared_memory_are_refused(cuda_lib):
             assert "too_large" in str(error), error
             refused.append(True)
     assert refused == sorted(refused) and not refused[0] and refused[-1]
+
+
+@pytest.mark.parametrize("multilabel", [False, True])
+def test_many_held_out_sets(cuda_lib, multilabel):
+    """Host arrays with more held-out sets than anybody would expect, each one's records its own."""
+    rng = np.random.default_rng(stable_seed("held out", multilabel))
+    n, d, m = 40, 6, 5
+    X, labels, offsets = random_problem(rng, n, d, m, np.float64, multilabel)
+    tests = []
+    for i in range(20):
+        Xi, li, oi = random_problem(rng, 10 + i, d, m, np.float64, multilabel)
+        tests.append((Xi, li, oi) if multilabel else (Xi, li))
+    A, W = np.zeros((n, m)), np.zeros((m, d))
+    objective = "mlsvm" if multilabel else "msvm"
+    out = cuda_lib.fit_(objective, X, labels, A, W=W, offsets=offsets, max_epoch=2, eval_epoch=1, tests=tests)
+    assert len(out["tests"]) == len(tests)
+    for got, t in zip(out["tests"], tests):
+        want = cuda_lib.evaluate(objective, t[0], t[1], W=W, offsets=t[2] if multilabel else None, is_train=False)
+        assert abs(got["primal_loss"][-1] - want["primal_loss"]) <= 1e-12 * max(1.0, want["primal_loss"])
