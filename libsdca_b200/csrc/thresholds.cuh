@@ -99,17 +99,42 @@ SDCAB_D void row_count_sum_gt(const Row& row, R cut, int& cnt, R& sum) {
 }
 
 // Ordered extraction: the entries already taken are those that precede
-// (v, idx) in the order "larger value first, smaller index first".
+// (v, idx) in the order "larger value first, smaller index first".  NaN is neither taken nor left.
 template <typename R>
 struct Taken {
   R v;
   int idx;
-  bool any;
-  SDCAB_HD Taken() : v(0), idx(-1), any(false) {}
-  SDCAB_HD bool has(R x, int i) const {
-    return any && (x > v || (x == v && i <= idx));
-  }
+  SDCAB_HD Taken() : v(num<R>::inf()), idx(-1) {}
+  SDCAB_HD bool has(R x, int i) const { return x > v || (x == v && i <= idx); }
+  SDCAB_HD bool left(R x, int i) const { return x < v || (x == v && i > idx); }
 };
+
+// The smallest index whose entry satisfies `pred` (INT_MAX: none does).
+template <typename R, typename Row, typename Pred>
+SDCAB_D int first_index(const Row& row, Pred pred) {
+  int first = INT_MAX;
+  row.for_each([&](typename Row::data_type xd, int i) {
+    if (i < first && pred(static_cast<R>(xd), i)) first = i;
+  });
+#if defined(SDCAB_WARP_GROUP)
+  first = __reduce_min_sync(kFullMask, first);
+#endif
+  return first;
+}
+
+// Largest value over the lanes and the smallest index that holds it; lanes without one carry (-inf,
+// INT_MAX).  No lane brings NaN, so all of them end with the same pair.
+template <typename R>
+SDCAB_D void warp_argmax(R& best, int& bi) {
+#if defined(SDCAB_WARP_GROUP)
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const R w = __shfl_xor_sync(kFullMask, best, o);
+    const int j = __shfl_xor_sync(kFullMask, bi, o);
+    if (w > best || (w == best && j < bi)) { best = w; bi = j; }
+  }
+#endif
+}
 
 // Takes the largest entry not yet taken; false if none is left.  NaN is never taken: no order holds
 // with it, and the lanes have to agree (warp_max).
@@ -119,20 +144,11 @@ SDCAB_D bool take_next(const Row& row, Taken<R>& tk, R& val) {
   int bi = INT_MAX;
   row.for_each([&](typename Row::data_type xd, int i) {
     R x = static_cast<R>(xd);
-    if (!tk.has(x, i) && (x > best || (bi == INT_MAX && x == x))) { best = x; bi = i; }
+    if (tk.left(x, i) && (bi == INT_MAX || x > best)) { best = x; bi = i; }
   });
-  // lanes without a candidate carry (-inf, INT_MAX) and lose every comparison
-#if defined(SDCAB_WARP_GROUP)
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    R w = __shfl_xor_sync(kFullMask, best, o);
-    int j = __shfl_xor_sync(kFullMask, bi, o);
-    bool take = (j != INT_MAX) && (bi == INT_MAX || w > best || (w == best && j < bi));
-    if (take) { best = w; bi = j; }
-  }
-#endif
+  warp_argmax(best, bi);
   if (bi == INT_MAX) return false;
-  tk.v = best; tk.idx = bi; tk.any = true;
+  tk.v = best; tk.idx = bi;
   val = best;
   return true;
 }
@@ -448,18 +464,11 @@ SDCAB_D void row_max_sumexp(const Row& row, Pred in, R& mx, R& s, int& count) {
     R x = static_cast<R>(xd);
     if (in(x, i)) {
       ++c;
-      if (x > best || (bi == INT_MAX && x == x)) { best = x; bi = i; }   // NaN as in take_next
+      if (x > best) { best = x; bi = i; }   // leaves NaN out, and -inf for now
     }
   });
-#if defined(SDCAB_WARP_GROUP)
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    R w = __shfl_xor_sync(kFullMask, best, o);
-    int j = __shfl_xor_sync(kFullMask, bi, o);
-    bool take = (j != INT_MAX) && (bi == INT_MAX || w > best || (w == best && j < bi));
-    if (take) { best = w; bi = j; }
-  }
-#endif
+  warp_argmax(best, bi);
+  if (bi == INT_MAX) bi = first_index<R>(row, [&](R x, int i) { return in(x, i) && x == -num<R>::inf(); });
   count = warp_sum(c);
   R acc = 0;
   row.for_each([&](typename Row::data_type xd, int i) {
