@@ -252,17 +252,20 @@ static EvalLayout eval_layout(long long n, long long m, long long elem, int sm_c
   EvalLayout L;
   const long long budget = 256LL << 20;
   long long chunk = std::max<long long>(128, budget / std::max<long long>(1, m * elem));
+  if (g_test_eval_chunk > 0) chunk = g_test_eval_chunk;
+  chunk = std::min(chunk, kMaxChunkRows);
+  // room for what the budget allows: a workspace sized for n examples is enough for fewer, although
+  // these may be evaluated in a longer chunk
+  const long long rows = std::min(chunk, std::max<long long>(n, 1));
+  L.scores_bytes = (static_cast<size_t>(rows) * m * elem + 255) & ~static_cast<size_t>(255);
   // Float scores in several chunks: whole rounds of the paired tensor-core kernel's 256 x 256 tiles
   // over the SM pairs, where that takes no more chunks (131 072 x 1000 classes: 28 rounds in two
   // chunks instead of 29).
   const long long pairs = std::max(1, sm_count / 2), col_tiles = (m + 255) / 256;
   const long long whole = (chunk / 256) * col_tiles / pairs * pairs / col_tiles * 256;
-  if (elem == 4 && n > chunk && whole > 0 && (n + whole - 1) / whole == (n + chunk - 1) / chunk) chunk = whole;
-  if (g_test_eval_chunk > 0) chunk = g_test_eval_chunk;
-  chunk = std::min(chunk, kMaxChunkRows);
-  chunk = std::min(chunk, std::max<long long>(n, 1));
-  L.chunk = chunk;
-  L.scores_bytes = (static_cast<size_t>(chunk) * m * elem + 255) & ~static_cast<size_t>(255);
+  if (elem == 4 && g_test_eval_chunk <= 0 && n > chunk && whole > 0 && (n + whole - 1) / whole == (n + chunk - 1) / chunk)
+    chunk = whole;
+  L.chunk = std::min(chunk, rows);
   L.max_blocks = std::max(1, sm_count) * 16;
   L.partials_bytes = (static_cast<size_t>(L.max_blocks) * 4 * sizeof(double) + 255) & ~static_cast<size_t>(255);
   L.hist_bytes = (static_cast<size_t>(m) * sizeof(unsigned long long) + 255) & ~static_cast<size_t>(255);

@@ -151,3 +151,14 @@ def test_a_shared_limit_is_never_lowered(hostsim):
     f = hostsim.lib.sdcab_hostsim_raise_limit
     f.restype = C.c_int64
     assert f(C.c_int(4), C.c_int(20000)) == 0
+
+
+def test_evaluation_workspace_of_more_examples_suffices_for_fewer():
+    """A caller sizes the workspace once, for the largest set it evaluates."""
+    query = b.lib()["sdcab_eval_workspace_bytes"]
+    query.restype = C.c_size_t
+    for m in (10, 257, 1000, 5000):
+        for item in (4, 8):
+            sizes = np.unique(np.concatenate([np.linspace(1, 5e8 / (m * item), 300), 2.0 ** np.arange(22)]).astype(int))
+            need = [query(C.c_int64(int(n)), C.c_int64(m), C.c_int64(item)) for n in sizes]
+            assert need == sorted(need), (m, item)
