@@ -1,4 +1,5 @@
-// Pieces shared by the kernels that walk through a block of SDCA steps (fit.cu, fit_entropy.cuh).
+// Pieces shared by the kernels that walk through a block of SDCA steps (fit_steps.cuh, fit_entropy.cuh)
+// and by their launches (fit.cu).
 #pragma once
 
 #include "update_core.cuh"

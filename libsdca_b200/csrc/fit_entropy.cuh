@@ -155,7 +155,7 @@ __device__ __forceinline__ bool solve_sum_w(int m, R alpha, SolverReduce& red, E
   return true;
 }
 
-// Steps b = 0 .. count - 1 as in fit_chain_kernel (fit.cu): four warps work the step, eight keep
+// Steps b = 0 .. count - 1 as in fit_chain_kernel (fit_steps.cuh): four warps work the step, eight keep
 // the later rows of S current and fetch the next step's variables and labels meanwhile.
 template <typename Data, typename R, bool ON_CHIP>
 __global__ void __launch_bounds__(kEntropyThreads, 1) fit_entropy_chain_kernel(ChainArgs p) {

@@ -131,7 +131,10 @@ int launch_rows(const Data* a, Data* out, int m, long long n, const ProxParams& 
   const int m_pad = (m + 15) & ~15;
   size_t smem = static_cast<size_t>(warps) * m_pad * sizeof(Data);
   int staged = 1;
-  // a copy of one row for each warp must leave room for the sixteen warps that registers allow
+  // A copy of one row for each warp must leave room for the sixteen warps that registers allow; longer
+  // rows are read through L1 and L2.  entropy_norm, read / copied: 1000 rows of 4000 floats 242 / 224 us,
+  // 600 of 12 000 748 / 1049, 600 of 14 000 doubles 1196 / 2028; biased top-k entropy 649 / 642, 1859 /
+  // 1830 and 2514 / 2826.
   const size_t room = kUneven ? info.smem_optin / 18 : info.smem_optin;
   if (smem > room) { staged = 0; smem = 0; }
   if (smem > 48 * 1024) {

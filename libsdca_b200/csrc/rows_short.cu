@@ -6,8 +6,9 @@
 // every thread runs the searches of thresholds.cuh on its own row with a group of one lane --
 // the rows sit an odd number of entries apart, so that the lanes of a warp read 32 different banks
 // -- and the block writes the mapped rows back.  Bound: instruction issue, m entries times the
-// passes of the slowest of 32 rows.  262 144 rows of 10 floats: knapsack 25 us against 210 us, top-k
-// cone (k = 5) 78 against 949 us, top-k entropy 76 against 891 us; rows_short.h has the limits.
+// passes of the slowest of 32 rows.  262 144 rows of 10 floats against one warp
+// per row: knapsack 30 / 117 us, top-k cone (k = 5) 71 / 798 us, top-k entropy 69 / 649 us; rows_short.h
+// has the limits.
 #define SDCAB_LANE_PER_ROW 1
 #include <algorithm>
 

@@ -11,18 +11,19 @@ template <typename Data>
 int launch_short_rows(int prox, const Data* a, Data* out, int m, long long n, const ProxParams& q,
                       cudaStream_t stream);
 
-// The longest rows for which one thread per row was faster than one warp per row at 262 144 rows
-// (k = 8 for the top-k operators), float and double data.  us, thread / warp, at the limit and one
-// size (8 or 16 entries) past it:
-//   knapsack            f32 48:  96 / 117, 64: 167 / 123      f64 32:  86 / 103, 40: 110 / 108
-//   knapsack_le         f32 48: 102 / 164, 64: 175 / 170      f64 40: 117 / 131, 48: 170 / 136
-//   knapsack_le_biased  f32 48: 110 / 183, 64: 182 / 169      f64 40: 126 / 178, 48: 182 / 153
-//   topk_simplex        f32 48: 200 / 248, 64: 265 / 247      f64 48: 244 / 359, 64: 384 / 359
-//   topk_simplex_biased f32 40: 673 / 920, 48: 742 / 715      f64 40: 660 / 1068, 48: 863 / 791
-//   topk_cone           f32 64: 260 / 345, 96: 301 / 233      f64 64: 350 / 415, 96: 432 / 324
-//   topk_cone_biased    f32 32: 402 / 1775, 40: 508 / 490     f64 32: 475 / 1739, 40: 613 / 507
-//   entropy             f32 48:  70 /  90, 64:  89 /  90      f64 64: 177 / 209, 96: 328 / 278
-//   topk_entropy        f32 32: 217 / 977, 40: 255 / 197      f64 64: 532 / 819, 96: 940 / 915
+// The longest rows that one thread per row takes, float and double data.  us at 262 144 rows (k = 8 for
+// the top-k operators), thread / warp, at the limit and one size past it:
+//   knapsack            f32 48:  88 / 125,  64: 144 / 130      f64 32:  76 / 113,  40:  92 / 116
+//   knapsack_le         f32 48:  93 / 171,  64: 150 / 178      f64 40:  96 / 140,  48: 131 / 141
+//   knapsack_le_biased  f32 48: 104 / 188,  64: 160 / 177      f64 40: 110 / 176,  48: 147 / 161
+//   topk_simplex        f32 48: 184 / 247,  64: 267 / 247      f64 48: 247 / 370,  64: 382 / 370
+//   topk_simplex_biased f32 40: 470 / 828,  48: 539 / 575      f64 40: 490 / 959,  48: 617 / 669
+//   topk_cone           f32 64: 202 / 305,  80: 224 / 242      f64 64: 253 / 415,  80: 331 / 372
+//   topk_cone_biased    f32 32: 298 / 1465, 40: 370 / 491      f64 32: 297 / 1421, 40: 379 / 506
+//   entropy             f32 48:  76 /  96,  64:  96 /  95      f64 64: 185 / 207,  80: 283 / 277
+//   topk_entropy        f32 32: 146 / 501,  40: 153 / 171      f64 64: 331 / 325,  80: 489 / 378
+// The lines were drawn where the thread stopped being faster before its searches took their cuts and
+// lost a comparison per entry: some could lie one size further out now.
 // The Lambert operators' rows differ too much in cost to share a warp.
 inline int short_row_limit(int prox, bool is_double) {
   switch (prox) {
@@ -39,8 +40,8 @@ inline int short_row_limit(int prox, bool is_double) {
 }
 
 // A thread's time grows with the row and does not shrink with the launch, so the fewer rows there
-// are, the shorter they have to be: knapsack of 32 floats took 28 us against a warp's 17 us at 16 384
-// rows and 61 against 108 us at 262 144.
+// are, the shorter they have to be: knapsack of 32 floats took 19 us against a warp's 18 us at 16 384
+// rows, 36 against 51 us at 98 304 and 59 against 115 us at 262 144.
 inline bool short_rows_usable(int prox, int m, long long n, bool is_double) {
   return m <= short_row_limit(prox, is_double) && n >= 3000LL * m;
 }

@@ -858,7 +858,7 @@ SDCAB_D Thr<R> thr_entropy_norm(const Row& row, R hi, R rhs) {
 // U would be accepted.
 template <typename R>
 __device__ __forceinline__ bool topk_entropy_newton_done(R s1, R s, R t1, R t, R cur, bool outputs_only) {
-  if (sizeof(R) != 8) return abs_(s1 - s) + abs_(t1 - t) <= 16 * num<R>::eps();
+  if (sizeof(R) != 8) return false;   // floats keep the reference's test alone
   if (abs_(s1 - s) + abs_(t1 - t) <= 16 * num<R>::eps() * max_(R(1), abs_(t))) return true;
   return outputs_only && s1 <= R(0) && s == R(0) && t > cur - R(5);
 }

@@ -46,6 +46,7 @@ def check(oracle, cuda_lib, name, a, precision, offset=0, **kw):
                                   "topk_entropy"])
 @pytest.mark.parametrize("dtype,precision", TYPES)
 def test_rows_off_the_vector_grid(oracle, cuda_lib, name, dtype, precision):
+    """Element-wise register rows (with float thresholds the general kernel, the same sizes)."""
     rng = np.random.default_rng(stable_seed("off-grid", name, str(dtype), precision))
     # one past / one short of each number of elements per lane, and even lengths on an odd base
     for m, offset in ((9, 0), (31, 0), (33, 1), (129, 0), (255, 0), (256, 1), (257, 0), (511, 0), (512, 1),
@@ -79,10 +80,12 @@ LONG = ["knapsack_eq", "knapsack_le", "knapsack_le_biased", "topk_simplex", "top
 @pytest.mark.parametrize("dtype,precision", TYPES)
 def test_long_rows(oracle, cuda_lib, name, dtype, precision):
     """Rows above the register kernels' limit, at the sizes where the block grows, where the copy no
-    longer fits shared memory, and off the vector grid."""
+    longer fits shared memory, and off the vector grid.  Doubles above 1024 entries and float thresholds
+    are the general kernel's at any length."""
     item = np.dtype(dtype).itemsize
     rng = np.random.default_rng(stable_seed("long", name, str(dtype), precision))
-    sizes = [(4096 // item + 1, 0), (1025, 1), (2048, 0), (16384 // item, 1), (16384 // item + 1, 0),
+    sizes = [(4096 // item + 1, 0), (1000 if item == 8 else 1027, 1), (1024 if item == 8 else 4095, 0), (1025, 1),
+             (2048, 0), (16384 // item, 1), (16384 // item + 1, 0),
              (57344 // item, 0), (57344 // item + 3, 1), (240000 // item, 1)]
     for m, offset in sizes:
         for kind in KINDS if m < 4000 else ("normal", "ties"):
@@ -125,7 +128,8 @@ def test_long_rows_repeat_bit_for_bit(cuda_lib, name, dtype, m):
 @pytest.mark.parametrize("dtype,precision", TYPES)
 def test_many_short_rows(oracle, cuda_lib, name, dtype, precision):
     """One thread per row: the lengths around the limits of the operators, the first row count that
-    takes the kernel and the last that does not, a last block that is not full."""
+    takes the kernel and the last that does not, a last block that is not full.  Float thresholds keep
+    one warp per row."""
     import torch
     rng = np.random.default_rng(stable_seed("short", name, str(dtype), precision))
     for m, n, offset in ((1, 3000, 0), (2, 6001, 1), (7, 21127, 0), (8, 23999, 0), (10, 30005, 1), (31, 93100, 0),
