@@ -854,13 +854,13 @@ SDCAB_D Thr<R> thr_entropy_norm(const Row& row, R hi, R rhs) {
 // past up to its limit of 32 iterations.  For |t| > 1 the last bits of t alone are above 16 eps:
 // the test has to be relative.  And an iteration that has reached s = 0 stays there (every term of
 // the next s has the factor s) while t grows by S0 / S1 <= 1 + W(exp(cur - t)), less than 7 a step
-// once t > cur - 5: what follows can neither change s nor bring t to cur + 708, where this size of
-// U would be accepted.
+// once t > cur - 5: below cur + 400 the steps that are left can neither change s nor bring t to
+// cur + 708, from where on this size of U is accepted.
 template <typename R>
 __device__ __forceinline__ bool topk_entropy_newton_done(R s1, R s, R t1, R t, R cur, bool outputs_only) {
   if (sizeof(R) != 8) return false;   // floats keep the reference's test alone
   if (abs_(s1 - s) + abs_(t1 - t) <= 16 * num<R>::eps() * max_(R(1), abs_(t))) return true;
-  return outputs_only && s1 <= R(0) && s == R(0) && t > cur - R(5);
+  return outputs_only && s1 <= R(0) && s == R(0) && t > cur - R(5) && t < cur + R(400);
 }
 #endif
 

@@ -154,3 +154,17 @@ def test_many_short_rows(oracle, cuda_lib, name, dtype, precision):
         else:
             ok, err = float_precision_ok(x, x_ref, oracle.prox(name, rows, result="double", **kw), rows, tol)
             assert ok, (name, m, kw, err)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_biased_topk_entropy_of_large_entries(oracle, cuda_lib, dtype):
+    """Rows in the hundreds and thousands, where the iteration for some sizes of U runs to s = 0 with t
+    far above the entries, and the reference accepts that."""
+    rng = np.random.default_rng(stable_seed("large entries", str(dtype)))
+    for m, k, alpha in ((15, 12, 4.0), (18, 12, 1.9), (22, 12, 3.6), (16, 5, 5.0), (40, 12, 4.3)):
+        a = (rng.standard_normal((6000, m)) * 10.0 ** rng.uniform(1, 4, (6000, 1))).astype(dtype)
+        kw = dict(k=k, alpha=alpha)
+        x = run_dev(cuda_lib, "topk_entropy_biased", a, 0, **kw)
+        # an entry's last bit is 1e-16 (double) or 6e-8 (float) of 1e4, and t and the outputs move with it
+        tol = 1e-9 if dtype == np.float64 else 1e-2
+        assert np.abs(x - oracle.prox("topk_entropy_biased", a, **kw)).max() <= tol, (m, k, alpha)
