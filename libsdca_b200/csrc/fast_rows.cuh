@@ -186,13 +186,13 @@ __device__ __forceinline__ T warp_sort_desc(T v, int lane) {
 }
 
 // Warp-wide maximum in one instruction (redux.sync on sm_100a handles f32;
-// doubles take the shuffle butterfly).
+// doubles take the shuffle butterfly, and must not be NaN).
 __device__ __forceinline__ float warp_max_fast(float v) {
   float r;
   asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
   return r;
 }
-__device__ __forceinline__ double warp_max_fast(double v) { return warp_max(v); }
+__device__ __forceinline__ double warp_max_fast(double v) { return warp_max_of_numbers(v); }
 
 // The (k+1)-th largest of the 32 lane values (k <= 31), counting repeats:
 // repeatedly take the warp maximum and retire the lanes that hold it.
@@ -201,6 +201,7 @@ __device__ __forceinline__ T kth_largest_of_lanes(T v, int k, int lane) {
   (void)lane;
   int seen = 0;
   T cur = v, top = -num<T>::inf();
+  if (sizeof(T) == 8 && !(v == v)) cur = top;   // the reduction of floats leaves NaN out itself
   for (int round = 0; round <= k; ++round) {
     top = warp_max_fast(cur);
     const unsigned hit = __ballot_sync(kFullMask, cur == top);

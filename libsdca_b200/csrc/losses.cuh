@@ -121,7 +121,7 @@ __device__ __forceinline__ float lanes_max(float v) {
   asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
   return r;
 }
-__device__ __forceinline__ double lanes_max(double v) { return warp_max(v); }
+__device__ __forceinline__ double lanes_max(double v) { return warp_max_of_numbers(v); }   // see topk_sums_device
 
 template <typename R, int K, typename Row>
 __device__ __forceinline__ void topk_sums_device(const Row& row, int k, R& sum_all, R& sum_pos) {

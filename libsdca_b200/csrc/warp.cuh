@@ -79,6 +79,19 @@ SDCAB_D int warp_sum(int v) {
 #endif
 }
 
+// The largest of the lanes' values, none of which may be NaN.
+template <typename T>
+SDCAB_D T warp_max_of_numbers(T v) {
+#if defined(SDCAB_WARP_GROUP)
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    T w = __shfl_xor_sync(kFullMask, v, o);
+    v = (w > v) ? w : v;
+  }
+#endif
+  return v;
+}
+
 // Maxima and minima leave NaN out (a group of nothing else gives the infinity of an empty one).  A
 // comparison with NaN is false from either side: the two lanes of an exchange would keep different
 // values, and lanes that disagree take different ways through loops with reductions in them, where they
@@ -87,13 +100,8 @@ template <typename T>
 SDCAB_D T warp_max(T v) {
 #if defined(SDCAB_WARP_GROUP)
   v = (v == v) ? v : static_cast<T>(-INFINITY);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    T w = __shfl_xor_sync(kFullMask, v, o);
-    v = (w > v) ? w : v;
-  }
 #endif
-  return v;
+  return warp_max_of_numbers(v);
 }
 
 template <typename T>
